@@ -368,8 +368,13 @@ __global__ void __launch_bounds__(TP_THREADS, 1)
                 const uint32_t s = 2 * i + h, sl = s % G::NR;
                 ok = tp_wait(&raw_full[sl], (s / G::NR) & 1);
                 if (!ok) continue;
-                if (h == 0) end = tiles[i % TP_RF].ph == TP_END;
-                if (end) continue;
+                if (h == 0) {
+                    end = tiles[i % TP_RF].ph == TP_END;
+                    // the end mark arrives on op_full too: not before tile i - NA's phase is over,
+                    // or it would stand in for a slower warp's operand
+                    if (end && i >= G::NA) ok = tp_wait(&op_empty[st], ((i / G::NA) - 1) & 1);
+                }
+                if (!ok || end) continue;
                 const uint32_t* src = reinterpret_cast<const uint32_t*>(raw + sl * TP_RAW) + 32 * q + lane;
                 uint32_t v[32];
 #pragma unroll
