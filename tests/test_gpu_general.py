@@ -162,6 +162,32 @@ def test_recover_random_k_of_2k(ctx, k):
         assert np.array_equal(got, data), (k, trial)
 
 
+# every length of a codeword, with and without the consistency check (which take different
+# passes), one column quad, a ragged width and one past a chunk of the scratch matrix
+@pytest.mark.parametrize("k", [1 << i for i in range(13)])
+def test_recover_every_length(ctx, k):
+    chunk = (64 << 20) // (2 * k)  # columns of the 256 MiB scratch matrix
+    for cols in (4, 132) + ((chunk + 36,) if k >= 256 else ()):
+        data = torch.randint(0, P, (k, cols), dtype=torch.int32, device="cuda",
+                             generator=torch.Generator(device="cuda").manual_seed(k + cols))
+        code = torch.empty((2 * k, cols), dtype=torch.int32, device="cuda")
+        ctx.extend(data, code, k, cols)
+        rng = np.random.default_rng(k * 7 + cols)
+        known = rng.permutation(2 * k)[:k]
+        known[0] |= 1  # an odd row, or the data rows might all be there
+        known = np.unique(known)
+        if len(known) < k:
+            known = np.append(known, np.setdiff1d(np.arange(2 * k), known)[:1])
+        lost = np.setdiff1d(np.arange(2 * k), known)
+        code[torch.from_numpy(lost).cuda()] = -1
+        for check in (False, True):
+            out = torch.full((k, cols), -1, dtype=torch.int32, device="cuda")
+            mm = ctx.recover(code, np.sort(known).tolist(), k, cols, out, check=check)
+            torch.cuda.synchronize()
+            assert torch.equal(out, data), (cols, check)
+            assert mm in (None, 0)
+
+
 def test_recover_matches_lagrange_oracle(ctx):
     k, cols = 32, 64
     data = O.seeded_input(k, cols, seed=9)

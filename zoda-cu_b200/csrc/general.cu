@@ -581,19 +581,20 @@ zoda_status zoda_recover_device(zoda_ctx* ctx, const uint32_t* d_code, const uin
     uint32_t* A = (uint32_t*)ctx->gen_a.p;
     // from the width at which the tensor-core passes win the extension of 2^ln rows, both
     // maps run there; the consistency count needs the coefficients, which they never form
-    const bool tensor = !mismatch && tensor_pays(ln, cols) && tensor_fits(ctx, ln, cols, st);
+    bool tensor = !mismatch && ln >= TENSOR_RECOVER_MIN_LOG && tensor_pays(ln, cols) && tensor_fits(ctx, ln, cols, st);
     if (tensor && (s = tensor_recover_tables(ctx, ln, zk, izh, T + 4 * N, st)) != ZODA_OK) return finish(s);
-    const bool tma = !tensor && ln >= DEC_TMA_MIN_LOG && ln <= DEC_TMA_MAX_LOG;
+    const bool tma = ln >= DEC_TMA_MIN_LOG && ln <= DEC_TMA_MAX_LOG;
     DecTables dt{};
-    if (tma && (s = dec_tables(ctx, ln, &dt)) != ZODA_OK) return finish(s);
     for (uint64_t c0 = 0; c0 < cols; c0 += w0) {
         const uint64_t w = std::min(w0, cols - c0);
         unsigned long long* cnt = mismatch ? d_cnt : nullptr;
         if (tensor) {
-            if ((s = tensor_recover(ctx, ln, d_code + c0, cols, T + 4 * N, A, d_data + c0, cols, w, st)) != ZODA_OK)
-                return finish(s);
-            continue;
+            s = tensor_recover(ctx, ln, d_code + c0, cols, T + 4 * N, A, d_data + c0, cols, w, st);
+            if (s == ZODA_OK) continue;
+            if (s != ZODA_ERR_UNSUPPORTED) return finish(s);
+            tensor = false;  // the fused passes take this chunk and the rest
         }
+        if (tma && !dt.ntt0_a && (s = dec_tables(ctx, ln, &dt)) != ZODA_OK) return finish(s);
         if (tma) {  // the same two passes on the TMA-staged shape
             if ((s = dec_pass(ctx, ln, false, dt, d_code + c0, cols, zk, A, w, w, nullptr, st)) != ZODA_OK)
                 return finish(s);

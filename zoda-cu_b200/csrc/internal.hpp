@@ -230,6 +230,7 @@ bool tensor_tables_host(int L, uint32_t base, bool lower_half, std::vector<uint8
 // The decoder on the passes, codewords of 2^11 and 2^12 rows, w columns at a time: `fac`
 // (16 bytes a row) filled once per erasure pattern, then a chunk's two launches. The
 // caller holds ctx->mu; scratch is [2^L][w].
+constexpr int TENSOR_RECOVER_MIN_LOG = 11;  // the one-CTA kernel of 1024 points takes no factors per row
 zoda_status tensor_recover_tables(zoda_ctx* ctx, int L, const uint2* zk, const uint2* izh, void* fac, cudaStream_t st);
 zoda_status tensor_recover(zoda_ctx* ctx, int L, const uint32_t* code, uint64_t code_pitch, const void* fac,
                            uint32_t* scratch, uint32_t* data, uint64_t data_pitch, uint64_t w,
