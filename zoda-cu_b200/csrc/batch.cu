@@ -85,7 +85,7 @@ constexpr uint64_t WIDE_MIN_COLS = 16384;
 bool leaves_queue(const zoda_ctx* ctx, const zoda_square& q) {
     const int L = log2_side(q.k);
     if (L != 10 && L != 11) return false;
-    if (L == 10 ? q.cols < WIDE_MIN_COLS : !tensor_pays(L, q.cols)) return false;
+    if (L == 10 ? q.cols < WIDE_MIN_COLS : !tensor_pays(ctx, L, q.cols, TensorUse::square)) return false;
     return q.cols < (1ull << 31) && ctx->impl == ZODA_IMPL_AUTO && (!ctx->planned[L] || is_tensor_plan(ctx->plan[L]));
 }
 zoda_status launch_alone(const zoda_ctx* ctx, const zoda_square& q, cudaStream_t st) {

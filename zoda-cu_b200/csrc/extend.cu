@@ -216,9 +216,12 @@ zoda_status launch_plan(const zoda_ctx* ctx, int log_s, const zoda_plan& p, cons
 zoda_status launch_extend(const zoda_ctx* ctx, int log_s, const uint32_t* in, uint32_t* out, uint64_t cols,
                           cudaStream_t st, int impl, bool odd_only, uint32_t in_rows, uint32_t out_rows) {
     if (log_s < 0 || log_s > 12) return ZODA_ERR_UNSUPPORTED;
+    const bool cut = in_rows && 4 * ((uint64_t)in_rows + out_rows) < (9ull << log_s);
+    const TensorUse use = cut ? TensorUse::cut : TensorUse::square;
     zoda_plan p = single_pass_plan(log_s);
     if (impl == ZODA_IMPL_AUTO && ctx->planned[log_s]) p = ctx->plan[log_s];
-    else if (impl == ZODA_IMPL_AUTO && (tensor_pays(log_s, cols) || log_s <= TENSOR_SMALL_MAX_LOG)) p = default_plan(log_s);
+    else if (impl == ZODA_IMPL_AUTO && (tensor_pays(ctx, log_s, cols, use) || log_s <= TENSOR_SMALL_MAX_LOG))
+        p = default_plan(log_s);
     else if (impl == ZODA_IMPL_DIRECT) p.impl = ZODA_IMPL_DIRECT;
     else if (impl == ZODA_IMPL_TMA) p.impl = ZODA_IMPL_TMA;
     else if (impl == ZODA_IMPL_FOURSTEP && log_s >= FOURSTEP_MIN_LOG) p.impl = ZODA_IMPL_FOURSTEP;

@@ -395,7 +395,7 @@ zoda_status encode_general(zoda_ctx* ctx, const uint32_t* in, uint32_t* out, uin
     // on the tensor cores every coset is one map, and coset 1's also writes coset 0: the rows
     // are in shared memory anyway (a separate copy of 1000 x 128000 takes 0.17 ms)
     if (R >= 2 && R <= (uint64_t)TENSOR_MAX_COSETS && lp >= TENSOR_MIN_LOG && lp <= TENSOR_MAX_LOG &&
-        tensor_pays(lp, cols) && tensor_fits(ctx, lp, cols, st) && m0 >= P_ / 2) {
+        tensor_pays(ctx, lp, cols, TensorUse::coset) && tensor_fits(ctx, lp, cols, st) && m0 >= P_ / 2) {
         bool fits = true;
         for (uint64_t c = 1; c < R && c < rows_out && fits; c++) {
             const uint32_t mc = (uint32_t)std::min<uint64_t>(P_, (rows_out - c + R - 1) / R);
@@ -581,7 +581,7 @@ zoda_status zoda_recover_device(zoda_ctx* ctx, const uint32_t* d_code, const uin
     uint32_t* A = (uint32_t*)ctx->gen_a.p;
     // from the width at which the tensor-core passes win the extension of 2^ln rows, both
     // maps run there; the consistency count needs the coefficients, which they never form
-    bool tensor = !mismatch && ln >= TENSOR_RECOVER_MIN_LOG && tensor_pays(ln, cols) && tensor_fits(ctx, ln, cols, st);
+    bool tensor = !mismatch && ln >= TENSOR_RECOVER_MIN_LOG && tensor_pays(ctx, ln, cols, TensorUse::square) && tensor_fits(ctx, ln, cols, st);
     if (tensor && (s = tensor_recover_tables(ctx, ln, zk, izh, T + 4 * N, st)) != ZODA_OK) return finish(s);
     const bool tma = ln >= DEC_TMA_MIN_LOG && ln <= DEC_TMA_MAX_LOG;
     DecTables dt{};

@@ -208,13 +208,23 @@ zoda_status long_recover(zoda_ctx* ctx, const uint32_t* d_code, const std::vecto
 constexpr int TENSOR_MIN_LOG = 10, TENSOR_MAX_LOG = 12;
 // Where the passes beat the single-pass kernels (three dependent passes cost about 24 us
 // however narrow the matrix is). Measured, tensor / single pass in us: 2048 at 4096
-// columns 56 / 48, at 6144 70 / 74, at 262144 2050 / 3270 (2470 / 3290 under the power
+// columns 56 / 48, at 6144 70 / 74, at 262144 2050 / 3270 (2250 / 3290 under the power
 // cap, which the passes reach and the single-pass kernel does not); 4096 at 4 columns
-// 26 / 33, at 1024 43 / 43, at 2048 58 / 83, at 524288 10800 / 20700 under the cap. Side
+// 25 / 35, 512 34 / 42, 1184 44 / 44, 2048 54 / 85, 524288 9560 / 20600 under the cap. Side
 // 1024 (one CTA a tile, tensorsq.cuh): 4 columns 14 / 23, 4096 23 / 25, 8192 39 / 43,
 // 16384 65 / 90, 131072 498 / 576 under the cap.
-inline bool tensor_pays(int L, uint64_t cols) {
-    return L == 10 || L == 12 || (L == 11 && (cols << L) >= (12ull << 20));
+// An encode cut well below the square (fewer than 3/4 of its rows in and out) spares the
+// single pass stores, the passes little; it takes rounds of 16 (2048) or 8 columns an SM
+// and steps up with each: 1100 + 1000 rows at 6400 columns 68 / 65, 8192 80 / 83; 2100 +
+// 2000 at 512 34 / 36, 768 37 / 36, 1184 43 / 36, 3000 + 2000 at 1184 43 / 40, 1188 43 / 73.
+// Cosets of 2100 + 9000 rows (three of 4096): 512 102 / 105, 640 106 / 105, 1184 129 / 111,
+// 1188 128 / 173; of 2048 from 6144 on as the square's (1100 + 3300: 193 / 234).
+enum class TensorUse { square, cut, coset };
+inline bool tensor_pays(const zoda_ctx* ctx, int L, uint64_t cols, TensorUse use) {
+    const uint64_t sm = (uint64_t)ctx->sm_count;
+    if (L == 12) return use == TensorUse::square || cols <= 512 || cols > 8 * sm;
+    if (L == 11) return use == TensorUse::cut ? cols > 3 * 16 * sm : cols >= 6144;
+    return L == 10;
 }
 // Whether a launch over `cols` columns can run on `st`: the counters suffice, and the
 // stream is not being captured (the passes share the context's buffers, ordered by an
