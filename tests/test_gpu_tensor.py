@@ -266,3 +266,12 @@ def test_tensor_encode_route_edges(ctx, k, n, fixed, per_sm, over):
     for c0 in (0, cols - 20):
         want = O.encode_rowmajor(np.ascontiguousarray(data[:, c0:c0 + 20]), n)
         assert np.array_equal(from_dev(out[:, c0:c0 + 20]), want)
+
+
+# the decoder on either side of the widths where its route changes: codewords of 2048 rows at
+# 6144 columns, of 4096 rows at 256 and at one round of the fused pass's tiles of 8 columns
+@pytest.mark.parametrize("over", [False, True])
+@pytest.mark.parametrize("k,fixed,per_sm", [(1024, 6140, 0), (2048, 256, 0), (2048, 0, 8)])
+def test_recover_route_edges(ctx, k, fixed, per_sm, over):
+    cols = fixed + per_sm * torch.cuda.get_device_properties(0).multi_processor_count + 4 * over
+    test_tensor_recover(ctx, k, cols)

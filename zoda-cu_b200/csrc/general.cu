@@ -579,9 +579,10 @@ zoda_status zoda_recover_device(zoda_ctx* ctx, const uint32_t* d_code, const uin
     const uint64_t w0 = chunk_cols(cols, N);
     if ((s = ctx->gen_a.ensure((uint64_t)N * w0 * 4)) != ZODA_OK) return finish(s);
     uint32_t* A = (uint32_t*)ctx->gen_a.p;
-    // from the width at which the tensor-core passes win the extension of 2^ln rows, both
-    // maps run there; the consistency count needs the coefficients, which they never form
-    bool tensor = !mismatch && ln >= TENSOR_RECOVER_MIN_LOG && tensor_pays(ctx, ln, cols, TensorUse::square) && tensor_fits(ctx, ln, cols, st);
+    // where the tensor-core passes are faster, both maps run there; the consistency count
+    // needs the coefficients, which they never form
+    bool tensor = !mismatch && ln >= TENSOR_RECOVER_MIN_LOG && tensor_pays(ctx, ln, cols, TensorUse::recover) &&
+                  tensor_fits(ctx, ln, cols, st);
     if (tensor && (s = tensor_recover_tables(ctx, ln, zk, izh, T + 4 * N, st)) != ZODA_OK) return finish(s);
     const bool tma = ln >= DEC_TMA_MIN_LOG && ln <= DEC_TMA_MAX_LOG;
     DecTables dt{};
