@@ -178,3 +178,26 @@ def test_rlc_check_matches_reference_validation(ctx):
     ok = O.validate_encoding(data, from_dev(code))
     assert ok[0] if isinstance(ok, tuple) else ok
     assert ctx.rlc_check(d_in, code, k, k, cols, coeff) == 0
+
+
+# device memory a call keeps for its coefficient tables: 16 bytes a column below 256 rows
+# (the few-rows kernel), 64 from there on, both only for a check that crosses the line
+@pytest.mark.parametrize("rows,per_col", [(8, 16), (256, 64)])
+def test_tables_hold_what_the_call_fills(rows, per_col):
+    import zoda_b200
+    cols = 1 << 20
+    x = torch.ones((rows, cols), dtype=torch.int32, device="cuda")
+    coeff = torch.ones((cols, 4), dtype=torch.int32, device="cuda")
+    out = torch.empty((rows, 4), dtype=torch.int32, device="cuda")
+    c = zoda_b200.Context(0)
+    try:
+        c.rlc_rows(x, rows, 32, coeff, out)  # what the first launch of the kernels loads
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        c.rlc_rows(x, rows, cols, coeff, out)
+        torch.cuda.synchronize()
+        kept = free - torch.cuda.mem_get_info()[0]
+        assert np.all(from_dev(out) == cols % P)
+    finally:
+        c.close()
+    assert kept <= per_col * cols + (8 << 20)

@@ -638,26 +638,30 @@ unsigned grid1(const zoda_ctx* ctx, uint64_t n) {
 // few-rows kernel (a thread per column quad).
 constexpr uint32_t RLC_ROW_KERNEL_MIN_ROWS = 256;
 
-// Byte offset of the digit table in ctx->rlc_w, after the planar one, and its row length.
-inline uint64_t digits_offset(uint64_t cols) { return (cols * 16 + 255) / 256 * 256; }
+// The tables of one call in ctx->rlc_w: 16 bytes a column where the few-rows kernel runs, 64
+// where the row kernel does.
+struct RlcTables {
+    const int4* planar;
+    const uint32_t* digits;
+};
+// Row length of the digit table.
 inline uint64_t digits_cols(uint64_t cols) { return (cols + rlct::BOX_C - 1) / rlct::BOX_C * rlct::BOX_C; }
 
 // rlc of rows [rows][cols] (pitch cols) into out [rows][4]; tables prepared.
-zoda_status rlc_rows(const zoda_ctx* ctx, const uint32_t* x, uint32_t rows, uint64_t cols, unsigned long long* acc,
-                     uint32_t* out, cudaStream_t st) {
+zoda_status rlc_rows(const zoda_ctx* ctx, const RlcTables& tabs, const uint32_t* x, uint32_t rows, uint64_t cols,
+                     unsigned long long* acc, uint32_t* out, cudaStream_t st) {
     ZB_CUDA(cudaMemsetAsync(acc, 0, (size_t)rows * 4 * sizeof(unsigned long long), st));
     const uint64_t quads = cols / 4;
     if (rows > 262140) {
         set_last_error_text("rlc: more than 262140 rows");
         return ZODA_ERR_UNSUPPORTED;
     }
-    const unsigned char* tabs = (const unsigned char*)ctx->rlc_w.p;
     if (quads && rows >= RLC_ROW_KERNEL_MIN_ROWS) {
         CUtensorMap tm_x, tm_c;
         const uint64_t npad = digits_cols(cols);
         zoda_status s = make_map(&tm_x, x, cols, rows, cols * 4, rlct::BOX_C, rlct::BOX_R, CU_TENSOR_MAP_SWIZZLE_128B);
         if (s == ZODA_OK)
-            s = make_map(&tm_c, tabs + digits_offset(cols), npad, 16, npad * 4, rlct::BOX_C, 16,
+            s = make_map(&tm_c, tabs.digits, npad, 16, npad * 4, rlct::BOX_C, 16,
                          CU_TENSOR_MAP_SWIZZLE_128B);
         if (s != ZODA_OK) return s;
         const uint64_t units = (cols + rlct::BOX_C - 1) / rlct::BOX_C * ((rows + rlct::UROWS - 1) / rlct::UROWS);
@@ -667,7 +671,7 @@ zoda_status rlc_rows(const zoda_ctx* ctx, const uint32_t* x, uint32_t rows, uint
     } else if (quads) {
         const uint64_t units = (quads + rlcb::CHQ - 1) / rlcb::CHQ * ((rows + rlcb::UROWS - 1) / rlcb::UROWS);
         const unsigned g = (unsigned)std::min<uint64_t>(units, (uint64_t)ctx->sm_count);
-        k_rlc_rows<<<g, rlcb::THREADS, rlcb::SMEM, st>>>(x, cols, rows, quads, (const int4*)tabs, acc, ctx->d_err);
+        k_rlc_rows<<<g, rlcb::THREADS, rlcb::SMEM, st>>>(x, cols, rows, quads, tabs.planar, acc, ctx->d_err);
         ZB_CUDA(cudaGetLastError());
     }
     k_rlc_final<<<grid1(ctx, (uint64_t)rows * 4), 256, 0, st>>>(acc, (uint64_t)rows * 4, out);
@@ -678,19 +682,18 @@ zoda_status rlc_rows(const zoda_ctx* ctx, const uint32_t* x, uint32_t rows, uint
 // Coefficient tables for RLCs of `rows_a` and `rows_b` rows (0: none): only the
 // layouts the kernels for those row counts read.
 zoda_status prep_tables(zoda_ctx* ctx, const uint32_t* d_coeff, uint64_t cols, uint32_t rows_a, uint32_t rows_b,
-                        cudaStream_t st) {
-    zoda_status s;
-    const uint64_t npad = digits_cols(cols);
-    if ((s = ctx->rlc_w.ensure(digits_offset(cols) + npad * 64)) != ZODA_OK) return s;
-    unsigned char* tabs = (unsigned char*)ctx->rlc_w.p;
+                        RlcTables* out, cudaStream_t st) {
     auto row_kernel = [](uint32_t r) { return r >= RLC_ROW_KERNEL_MIN_ROWS; };
     const bool planar = (rows_a && !row_kernel(rows_a)) || (rows_b && !row_kernel(rows_b));
     const bool digits = row_kernel(rows_a) || row_kernel(rows_b);
+    const uint64_t npad = digits_cols(cols), at = planar ? (cols * 16 + 255) / 256 * 256 : 0;
+    zoda_status s;
+    if ((s = ctx->rlc_w.ensure(at + (digits ? npad * 64 : 0))) != ZODA_OK) return s;
+    unsigned char* w = (unsigned char*)ctx->rlc_w.p;
+    *out = RlcTables{(const int4*)w, (const uint32_t*)(w + at)};
     if (cols == 0) return ZODA_OK;
-    if (planar) k_rlc_prep<<<grid1(ctx, cols), 256, 0, st>>>((const uint4*)d_coeff, cols / 4, (int4*)tabs);
-    if (digits)
-        k_rlc_digits<<<grid1(ctx, npad), 256, 0, st>>>((const uint4*)d_coeff, cols, npad,
-                                                       (uint32_t*)(tabs + digits_offset(cols)));
+    if (planar) k_rlc_prep<<<grid1(ctx, cols), 256, 0, st>>>((const uint4*)d_coeff, cols / 4, (int4*)w);
+    if (digits) k_rlc_digits<<<grid1(ctx, npad), 256, 0, st>>>((const uint4*)d_coeff, cols, npad, (uint32_t*)(w + at));
     ZB_CUDA(cudaGetLastError());
     return ZODA_OK;
 }
@@ -775,10 +778,11 @@ zoda_status zoda_rlc_rows_device(zoda_ctx* ctx, const uint32_t* d_rows, uint32_t
     ZB_CUDA(cudaSetDevice(ctx->device));
     cudaStream_t st = (cudaStream_t)stream;
     std::lock_guard<std::mutex> lock(ctx->rlc_mu);
-    zoda_status s = prep_tables(ctx, d_coeff, cols, rows, 0, st);
+    RlcTables tabs{};
+    zoda_status s = prep_tables(ctx, d_coeff, cols, rows, 0, &tabs, st);
     if (s != ZODA_OK) return s;
     if ((s = ctx->rlc_acc.ensure((size_t)rows * 4 * 8)) != ZODA_OK) return s;
-    return rlc_rows(ctx, d_rows, rows, cols, (unsigned long long*)ctx->rlc_acc.p, d_out, st);
+    return rlc_rows(ctx, tabs, d_rows, rows, cols, (unsigned long long*)ctx->rlc_acc.p, d_out, st);
 }
 
 zoda_status zoda_rlc_check_device(zoda_ctx* ctx, const uint32_t* d_data, const uint32_t* d_code, uint32_t k,
@@ -790,7 +794,8 @@ zoda_status zoda_rlc_check_device(zoda_ctx* ctx, const uint32_t* d_data, const u
     cudaStream_t st = (cudaStream_t)stream;
     const uint32_t rows = k + n;
     std::lock_guard<std::mutex> lock(ctx->rlc_mu);
-    zoda_status s = prep_tables(ctx, d_coeff, cols, k, rows, st);
+    RlcTables tabs{};
+    zoda_status s = prep_tables(ctx, d_coeff, cols, k, rows, &tabs, st);
     if (s != ZODA_OK) return s;
     if ((s = ctx->rlc_acc.ensure((size_t)rows * 4 * 8)) != ZODA_OK) return s;
     if ((s = ctx->rlc_d.ensure((size_t)k * 16)) != ZODA_OK) return s;
@@ -799,10 +804,10 @@ zoda_status zoda_rlc_check_device(zoda_ctx* ctx, const uint32_t* d_data, const u
     if ((s = ctx->rlc_cnt.ensure(8)) != ZODA_OK) return s;
     unsigned long long* acc = (unsigned long long*)ctx->rlc_acc.p;
     uint32_t *D = (uint32_t*)ctx->rlc_d.p, *E = (uint32_t*)ctx->rlc_e.p, *F = (uint32_t*)ctx->rlc_f.p;
-    if ((s = rlc_rows(ctx, d_data, k, cols, acc, D, st)) != ZODA_OK) return s;
+    if ((s = rlc_rows(ctx, tabs, d_data, k, cols, acc, D, st)) != ZODA_OK) return s;
     // the RLC and the extension commute (both F_p-linear): extend the k x 4 RLC matrix
     if ((s = zoda_encode_device(ctx, D, F, k, n, 4, st)) != ZODA_OK) return s;
-    if ((s = rlc_rows(ctx, d_code, rows, cols, acc, E, st)) != ZODA_OK) return s;
+    if ((s = rlc_rows(ctx, tabs, d_code, rows, cols, acc, E, st)) != ZODA_OK) return s;
     ZB_CUDA(cudaMemsetAsync(ctx->rlc_cnt.p, 0, 8, st));
     k_count_diff<<<grid1(ctx, (uint64_t)rows * 4), 256, 0, st>>>(E, F, (uint64_t)rows * 4,
                                                                 (unsigned long long*)ctx->rlc_cnt.p);
