@@ -101,3 +101,30 @@ def test_pipelined_fourstep_wait_runs_out_and_the_context_survives():
     finally:
         c.plan_clear()
         c.close()
+
+
+def test_context_without_room_for_the_ring():
+    """A device with less free memory than the tensor-core passes' ring takes: the context
+    is created all the same and a square of 4096 rows runs on the single-pass kernel."""
+    import zoda_b200
+    k, cols = 4096, 64
+    data = torch.from_numpy(O.seeded_input(k, cols, seed=3).view(np.int32)).cuda()
+    want = torch.empty((2 * k, cols), dtype=torch.int32, device="cuda")
+    got = torch.full((2 * k, cols), -1, dtype=torch.int32, device="cuda")
+    full = zoda_b200.Context(0)
+    small, hold = None, []
+    try:
+        full.extend(data, want, k, cols)
+        torch.cuda.synchronize()
+        while torch.cuda.mem_get_info()[0] > 64 << 20:
+            hold.append(torch.empty(torch.cuda.mem_get_info()[0] - (56 << 20), dtype=torch.uint8, device="cuda"))
+        small = zoda_b200.Context(0)
+        small.extend(data, got, k, cols)
+        small.check()
+        assert torch.equal(got, want)
+    finally:
+        hold.clear()
+        torch.cuda.empty_cache()
+        for c in (small, full):
+            if c:
+                c.close()
