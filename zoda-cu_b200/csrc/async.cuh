@@ -55,11 +55,6 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
         "l"(map), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
         : "memory");
 }
-__device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, int x, int y, int z, const void* src) {
-    asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%1, %2, %3}], [%4];" ::"l"(map), "r"(x),
-                 "r"(y), "r"(z), "r"(smem_u32(src))
-                 : "memory");
-}
 // The same with an L2 policy, e.g. for data touched once beside data that should stay.
 __device__ __forceinline__ uint64_t l2_evict_first() {
     uint64_t p;

@@ -65,13 +65,6 @@ std::vector<zoda_plan> candidates(int ls) {
         c.push_back(p);
     };
     add(single_pass_plan(ls));
-    if (ls >= TENSOR_MIN_LOG) {
-        zoda_plan p = d;
-        p.impl = ZODA_IMPL_FOURSTEP;
-        p.blocked = 1;
-        p.stagger = 0;
-        add(p);
-    }
     for (int blocked = 0; blocked <= 1; blocked++) {
         for (int radix : {16, 8}) {
             if (radix == 8 && ls < 6) continue;

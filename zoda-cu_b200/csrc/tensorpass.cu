@@ -25,14 +25,12 @@ constexpr uint64_t TENSOR_COUNTERS = 1 << 18;  // bytes: 3 counts a chunk
 
 // Rounds between a chunk's passes, and the ring's slots: a slot is reused that many rounds
 // after the last read of the chunk before it.
-template <class G>
-uint64_t pipe_depth(const zoda_ctx* ctx, uint64_t grid, uint64_t per_round) {
-    (void)ctx;
+uint64_t pipe_depth(uint64_t grid, uint64_t per_round) {
     return std::max<uint64_t>(1, ((uint64_t)ZB_TENSOR_HELD * grid + per_round - 1) / per_round);
 }
 template <class G>
 size_t ring_bytes(const zoda_ctx* ctx) {  // the widest launch: full grid, fewest items a round
-    const uint64_t d = pipe_depth<G>(ctx, (uint64_t)ctx->sm_count, G::TA + G::TM + G::TA / 2);
+    const uint64_t d = pipe_depth((uint64_t)ctx->sm_count, G::TA + G::TM + G::TA / 2);
     return (size_t)(3 * d + 1) * G::SLOT * 4;
 }
 
@@ -141,7 +139,7 @@ zoda_status launch_t(zoda_ctx* ctx, TensorArgs a, uint64_t cols, cudaStream_t st
     const uint64_t nch = (cols + G::CW - 1) / G::CW;
     const uint64_t per_round = G::TA + G::TM + (G::TA >> OSH);
     const uint64_t grid = std::min<uint64_t>((uint64_t)ctx->sm_count, nch * per_round);
-    const uint64_t depth = pipe_depth<G>(ctx, grid, per_round);
+    const uint64_t depth = pipe_depth(grid, per_round);
     if (cols >= (1ull << 31) || (nch + 2 * depth) * per_round + 16 * grid >= (1ull << 31)) return ZODA_ERR_UNSUPPORTED;
     a.nchunks = (uint32_t)nch;
     a.depth = (uint32_t)depth;
