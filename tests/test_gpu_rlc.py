@@ -201,3 +201,19 @@ def test_tables_hold_what_the_call_fills(rows, per_col):
     finally:
         c.close()
     assert kept <= per_col * cols + (8 << 20)
+
+
+# a check with the data below RLC's 256 rows and the code above: both coefficient tables,
+# widths around a thread block's and the row kernel's 32 columns
+@pytest.mark.parametrize("k,n", [(255, 1), (130, 300)])
+@pytest.mark.parametrize("cols", [4, 36, 252, 260, 2508])
+def test_rlc_check_across_the_kernels_line(ctx, k, n, cols):
+    data = O.seeded_input(k, cols, seed=k + cols)
+    code = torch.empty((k + n, cols), dtype=torch.int32, device="cuda")
+    d_in = to_dev(data)
+    ctx.encode(d_in, code, k, n, cols)
+    rng = np.random.default_rng(cols)
+    coeff = to_dev(rng.integers(0, 1 << 32, size=(cols, 4), dtype=np.uint64).astype(np.uint32))  # any u32
+    assert ctx.rlc_check(d_in, code, k, n, cols, coeff) == 0
+    code[k + n - 1, cols - 1] = (int(code[k + n - 1, cols - 1]) + 1) % P
+    assert ctx.rlc_check(d_in, code, k, n, cols, coeff) == 4

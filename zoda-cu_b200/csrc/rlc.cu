@@ -591,13 +591,16 @@ __global__ void __launch_bounds__(rlct::THREADS, 1)
 // per column and limb, its four residues independent products: a narrow matrix waits for
 // one thread's chain. With a thread per column and each residue made from the one before,
 // a call on 256 x 512 took 1.8 us more than the sums as multiply-adds (13.1), now 0.6.
+// With `planar`, the few-rows kernel's table too: a check with a matrix on either side of
+// RLC_ROW_KERNEL_MIN_ROWS makes both in one launch.
 __global__ void k_rlc_digits(const uint32_t* __restrict__ coeff, uint64_t cols, uint64_t npad,
-                             uint32_t* __restrict__ tab) {
+                             uint32_t* __restrict__ tab, int32_t* __restrict__ planar) {
     constexpr uint32_t shift[4] = {1u, 1u << 8, 1u << 16, 1u << 24};  // all below p
     const uint32_t l = blockIdx.y;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < npad;
          i += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t c = i < cols ? coeff[4 * i + l] : 0;  // any u32
+        if (planar && i < cols) planar[4 * ((i & 3) * (cols / 4) + (i >> 2)) + l] = centered(c % P);
         uint32_t w[4];
 #pragma unroll
         for (int y = 0; y < 4; y++) w[y] = balanced_digits(mul_slow(c, shift[y]));
@@ -689,9 +692,10 @@ zoda_status prep_tables(zoda_ctx* ctx, const uint32_t* d_coeff, uint64_t cols, u
     unsigned char* w = (unsigned char*)ctx->rlc_w.p;
     *out = RlcTables{(const int4*)w, (const uint32_t*)(w + at)};
     if (cols == 0) return ZODA_OK;
-    if (planar) k_rlc_prep<<<grid1(ctx, cols), 256, 0, st>>>((const uint4*)d_coeff, cols / 4, (int4*)w);
+    if (planar && !digits) k_rlc_prep<<<grid1(ctx, cols), 256, 0, st>>>((const uint4*)d_coeff, cols / 4, (int4*)w);
     if (digits)
-        k_rlc_digits<<<dim3(grid1(ctx, npad), 4), 256, 0, st>>>(d_coeff, cols, npad, (uint32_t*)(w + at));
+        k_rlc_digits<<<dim3(grid1(ctx, npad), 4), 256, 0, st>>>(d_coeff, cols, npad, (uint32_t*)(w + at),
+                                                                planar ? (int32_t*)w : nullptr);
     ZB_CUDA(cudaGetLastError());
     return ZODA_OK;
 }
