@@ -252,10 +252,10 @@ def test_server_wide_squares(ctx, shapes):
         srv.close()
 
 
-# encodes on either side of the widths where their route changes: 512 columns, and one round
+# encodes on either side of the widths where their route changes: 512 columns (cosets 256), and one round
 # of the single pass's tiles of 8 columns (4096) or three of 16 (2048)
 @pytest.mark.parametrize("over", [False, True])
-@pytest.mark.parametrize("k,n,fixed,per_sm", [(2100, 2000, 512, 0), (2100, 2000, 0, 8), (2100, 9000, 512, 0),
+@pytest.mark.parametrize("k,n,fixed,per_sm", [(2100, 2000, 512, 0), (2100, 2000, 0, 8), (2100, 9000, 256, 0),
                                               (2100, 9000, 0, 8), (1100, 1000, 0, 48)])
 def test_tensor_encode_route_edges(ctx, k, n, fixed, per_sm, over):
     cols = fixed + per_sm * torch.cuda.get_device_properties(0).multi_processor_count + 4 * over

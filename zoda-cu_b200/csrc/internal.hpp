@@ -217,15 +217,16 @@ constexpr int TENSOR_MIN_LOG = 10, TENSOR_MAX_LOG = 12;
 // single pass stores, the passes little; it takes rounds of 16 (2048) or 8 columns an SM
 // and steps up with each: 1100 + 1000 rows at 6400 columns 68 / 65, 8192 80 / 83; 2100 +
 // 2000 at 512 34 / 36, 768 37 / 36, 1184 43 / 36, 3000 + 2000 at 1184 43 / 40, 1188 43 / 73.
-// Cosets of 2100 + 9000 rows (three of 4096): 512 102 / 105, 640 106 / 105, 1184 129 / 111,
-// 1188 128 / 173; of 2048 from 6144 on as the square's (1100 + 3300: 193 / 234).
+// Three cosets of 4096: 2100 + 9000 rows at 256 columns 87 / 101, 512 102 / 105, 640 106 /
+// 105, 1184 129 / 111, 1188 128 / 173, 3600 + 4680 (half of their rows cut) at 256 86 / 90,
+// 512 103 / 92, 1188 128 / 164; of 2048 from 6144 on as the square's (1100 + 3300: 193 / 234).
 // The decoder, per call, against its two fused passes, which write no even rows: codewords of
 // 2048 at 6144 columns 158 / 174, 65536 971 / 1307; of 4096 at 4 95 / 105, 256 102 / 106, 384
 // 108 / 106, 512 112 / 106, 1184 132 / 107, 1188 132 / 155, 65536 2150 / 3170.
 enum class TensorUse { square, cut, coset, recover };
 inline bool tensor_pays(const zoda_ctx* ctx, int L, uint64_t cols, TensorUse use) {
     const uint64_t sm = (uint64_t)ctx->sm_count;
-    if (L == 12) return use == TensorUse::square || cols <= (use == TensorUse::recover ? 256 : 512) || cols > 8 * sm;
+    if (L == 12) return use == TensorUse::square || cols <= (use == TensorUse::cut ? 512 : 256) || cols > 8 * sm;
     if (L == 11) return use == TensorUse::cut ? cols > 3 * 16 * sm : cols >= 6144;
     return L == 10;
 }
