@@ -353,7 +353,9 @@ def time_recover(ctx, k: int, reps: int = 5, seed: int = 3) -> dict:
     torch.cuda.empty_cache()
     return {"k": k, "cols": cols, "erased_rows": k, "ms": round(ms, 4),
             "gbps": round(payload_bits(k) / (ms * 1e-3) / 1e9, 1), "bit_exact": ok,
-            "api": "zoda_recover_device (two fused passes, each an INTT and an NTT over 2k points, TMA-staged)"}
+            "api": "zoda_recover_device (two maps over 2k points, " +
+                   ("each three passes on the tensor cores)" if 2 * k in (2048, 4096)
+                    else "each one fused pass of an INTT and an NTT)")}
 
 
 def time_rlc(ctx, k: int, reps: int = 5) -> dict:
@@ -421,7 +423,9 @@ def time_encode_general(ctx, k: int, n: int, reps: int = 5) -> dict:
     del d_in, d_out
     torch.cuda.empty_cache()
     if r == 2:
-        api = "zoda_encode_device (n_kn = 2 n_k: the fused kernels, zeros past row k, output cut at k+n)"
+        api = "zoda_encode_device (n_kn = 2 n_k: the square's kernels, zeros past row k, output cut at k+n)"
+    elif 1024 <= n_k <= 4096 and r <= 16:
+        api = f"zoda_encode_device (n_kn = {r} n_k: one map on the tensor cores per coset, {r - 1} maps)"
     elif 128 <= n_k <= 4096:
         api = f"zoda_encode_device (n_kn = {r} n_k: one fused TMA-staged INTT + NTT pass per coset, {r - 1} passes)"
     else:

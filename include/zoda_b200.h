@@ -106,8 +106,9 @@ zoda_status zoda_ctx_set_impl(zoda_ctx* ctx, int impl);
  * (TMA for 128 <= k <= 2048, else direct; sched 0, l2_promo 3, blocked 0,
  * stagger 1, radix 16; sides 32 and 64: DIRECT with stagger 0; squares of 1024 and
  * 4096 rows and wide ones of 2048: FOURSTEP with blocked 1 and stagger 0, from 2048 rows
- * on the TMA or direct plan in a captured stream). Every plan computes the same bits; only the speed
- * differs. */
+ * on the TMA or direct plan in a captured stream, in a context created with too little
+ * device memory left for the passes' ring, and at some widths of encodes cut well below
+ * the square). Every plan computes the same bits; only the speed differs. */
 typedef struct zoda_plan {
     int32_t impl;     /* ZODA_IMPL_DIRECT, ZODA_IMPL_TMA (k >= 32) or ZODA_IMPL_FOURSTEP
                          (1024 <= k <= 4096)                                          */

@@ -208,9 +208,9 @@ zoda_status long_recover(zoda_ctx* ctx, const uint32_t* d_code, const std::vecto
 constexpr int TENSOR_MIN_LOG = 10, TENSOR_MAX_LOG = 12;
 // Where the passes beat the single-pass kernels (three dependent passes cost about 24 us
 // however narrow the matrix is). Measured, tensor / single pass in us: 2048 at 4096
-// columns 56 / 48, at 6144 70 / 74, at 262144 2050 / 3270 (2250 / 3290 under the power
+// columns 56 / 48, at 6144 70 / 74, at 262144 2050 / 3270 (2280 / 3300 under the power
 // cap, which the passes reach and the single-pass kernel does not); 4096 at 4 columns
-// 25 / 35, 512 34 / 42, 1184 44 / 44, 2048 54 / 85, 524288 9560 / 20600 under the cap. Side
+// 25 / 35, 512 34 / 42, 1184 44 / 44, 2048 54 / 85, 524288 9800 / 20700 under the cap. Side
 // 1024 (one CTA a tile, tensorsq.cuh): 4 columns 14 / 23, 4096 23 / 25, 8192 39 / 43,
 // 16384 65 / 90, 131072 498 / 576 under the cap.
 // An encode cut well below the square (fewer than 3/4 of its rows in and out) spares the

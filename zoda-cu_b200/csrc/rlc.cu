@@ -634,8 +634,9 @@ unsigned grid1(const zoda_ctx* ctx, uint64_t n) {
     return (unsigned)(g < 1 ? 1 : g > cap ? cap : g);
 }
 
-// From this many rows on, the row kernel (a thread per row) runs; below, the
-// few-rows kernel (a thread per column quad).
+// From this many rows on, the row kernel (the product on the tensor cores) runs; below,
+// the few-rows kernel (a thread per column quad). At 255 / 256 rows a call takes 15.5 /
+// 16.0 us at 512 columns and 47.9 / 43.7 at 131072.
 constexpr uint32_t RLC_ROW_KERNEL_MIN_ROWS = 256;
 
 // The tables of one call in ctx->rlc_w: 16 bytes a column where the few-rows kernel runs, 64

@@ -38,10 +38,10 @@
 //
 // What bounds it: the card's power limit. In a burst (1.9 GHz) a 4096 square takes 9.1 ms
 // and the instruction issue of the read-back is nearest its limit; under the 1000 W cap
-// the SM clock settles near 1.5 GHz and it takes 9.97 ms, 2.6 TB/s of the 12 bytes a value
-// that must move (the butterfly passes: 12.6 ms, the single pass 20.7). 2048: 2.31 ms
-// against 3.29. A tile's products take 1024 of its about 3000 cycles (64 points), its
-// HBM traffic is the 12 bytes a value plus a sixth more for ring lines that leave L2.
+// the SM clock settles near 1.5 GHz and it takes 9.6 .. 9.9 ms, 2.65 TB/s of the 12 bytes a
+// value that must move (the butterfly passes: 12.6 ms, the single pass 20.7). 2048: 2.26 ..
+// 2.30 ms against 3.29. A tile's products take 1024 of its about 3000 cycles (64 points), its
+// HBM traffic is the 12 bytes a value plus 27% for ring lines that leave L2.
 #pragma once
 #include "dft.cuh"
 #include "tcgen05.cuh"
