@@ -5,6 +5,7 @@
 // test_tensor_roles.py removes its inline-PTX helpers, which are restated here.
 #include <ucontext.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <cstdio>
 #include <cstdlib>
